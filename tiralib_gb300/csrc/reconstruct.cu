@@ -143,7 +143,8 @@ __global__ void __launch_bounds__(256) k_otsu(const unsigned long long* __restri
     const double mu0 = w0 > 0.0 ? prod[i] / w0 : 0.0;
     const double mu1 = w1 > 0.0 ? (cum_all - prod[i]) / w1 : 0.0;
     const double dm = mu0 - mu1;
-    var[i] = (w0 * w1) * (dm * dm);
+    const double bv = (w0 * w1) * (dm * dm);
+    var[i] = bv > -1.0 ? bv : -1.0;                        // an infinite range makes it NaN, which never wins
     at[i] = i;
     __syncthreads();
     for (int o = 128; o > 0; o >>= 1) {
@@ -153,7 +154,7 @@ __global__ void __launch_bounds__(256) k_otsu(const unsigned long long* __restri
         }
         __syncthreads();
     }
-    if (i == at[0]) *thr = c;
+    if (i == at[0]) *thr = var[0] > -1.0 ? c : 0.0;
 }
 
 // s > thr with the threshold in FP64, as NumPy compares a float32 map with a Python float
