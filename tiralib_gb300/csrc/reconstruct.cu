@@ -265,29 +265,31 @@ template <class I>
 __global__ void __launch_bounds__(256) k_uf_init(const unsigned char* __restrict__ fg, I* __restrict__ p, int H, int W) {
     const int lane = threadIdx.x, x = blockIdx.x * 32 + lane;
     if (blockIdx.x == 0 && blockIdx.y == 0 && lane == 0 && threadIdx.y == 0) p[0] = 0;
-    const int y = blockIdx.y * 8 + threadIdx.y;
-    if (y >= H) return;
-    const bool bg = x < W && !fg[size_t(y) * W + x];
-    const unsigned runs = __ballot_sync(0xffffffffu, bg);
-    if (x >= W) return;
-    const size_t i = size_t(y) * W + x;
-    const unsigned below = ~runs & ((1u << lane) - 1u);    // foreground to the left, within the warp
-    const int start = below ? 32 - __clz(below) : 0;
-    const bool border = x == 0 || y == 0 || x == W - 1 || y == H - 1;
-    p[i + 1] = I(bg ? (border ? 0 : i + 1 - (lane - start)) : i + 1);
+    for (int y = blockIdx.y * 8 + threadIdx.y; y < H; y += gridDim.y * 8) {   // the same rows for a whole warp
+        const bool bg = x < W && !fg[size_t(y) * W + x];
+        const unsigned runs = __ballot_sync(0xffffffffu, bg);
+        if (x >= W) continue;
+        const size_t i = size_t(y) * W + x;
+        const unsigned below = ~runs & ((1u << lane) - 1u);   // foreground to the left, within the warp
+        const int start = below ? 32 - __clz(below) : 0;
+        const bool border = x == 0 || y == 0 || x == W - 1 || y == H - 1;
+        p[i + 1] = I(bg ? (border ? 0 : i + 1 - (lane - start)) : i + 1);
+    }
 }
 template <class I>
 __global__ void __launch_bounds__(256) k_uf_link(const unsigned char* __restrict__ fg, I* __restrict__ p, int H, int W) {
-    const int x = blockIdx.x * 32 + threadIdx.x, y = blockIdx.y * 8 + threadIdx.y;
-    if (x >= W || y >= H) return;
-    const size_t i = size_t(y) * W + x;
-    if (fg[i]) return;
-    const bool left = x > 0 && !fg[i - 1], up = y > 0 && !fg[i - W];
-    const bool border = x == 0 || y == 0 || x == W - 1 || y == H - 1;
-    // runs meet across warps; a border pixel's parent is the outside, so its run is linked here too
-    if (left && ((x & 31) == 0 || border || x == 1 || y == 0 || y == H - 1)) uf_link(p, I(i + 1), I(i));
-    // one link per stretch of pixels whose upper neighbours are background too
-    if (up && !(left && !fg[i - W - 1])) uf_link(p, I(i + 1), I(i + 1 - W));
+    const int x = blockIdx.x * 32 + threadIdx.x;
+    if (x >= W) return;
+    for (int y = blockIdx.y * 8 + threadIdx.y; y < H; y += gridDim.y * 8) {
+        const size_t i = size_t(y) * W + x;
+        if (fg[i]) continue;
+        const bool left = x > 0 && !fg[i - 1], up = y > 0 && !fg[i - W];
+        const bool border = x == 0 || y == 0 || x == W - 1 || y == H - 1;
+        // runs meet across warps; a border pixel's parent is the outside, so its run is linked here too
+        if (left && ((x & 31) == 0 || border || x == 1 || y == 0 || y == H - 1)) uf_link(p, I(i + 1), I(i));
+        // one link per stretch of pixels whose upper neighbours are background too
+        if (up && !(left && !fg[i - W - 1])) uf_link(p, I(i + 1), I(i + 1 - W));
+    }
 }
 template <class I>
 __global__ void __launch_bounds__(256) k_uf_finish(const unsigned char* __restrict__ fg, I* __restrict__ p, size_t n,
@@ -470,9 +472,10 @@ int tvgb_saliency_threshold2(const float* field, unsigned s0, unsigned s1, int f
         }
         auto fill_holes = [&](auto* parent) -> int {
             KernelTimer kt_("k_fill", st);
-            k_uf_init<<<g, blk, 0, st>>>(cur, parent, H, W);
+            const dim3 gu(g.x, std::min(g.y, 65535u));        // taller images: several rows per thread
+            k_uf_init<<<gu, blk, 0, st>>>(cur, parent, H, W);
             TVGB_LAUNCHED();
-            k_uf_link<<<g, blk, 0, st>>>(cur, parent, H, W);
+            k_uf_link<<<gu, blk, 0, st>>>(cur, parent, H, W);
             TVGB_LAUNCHED();
             k_uf_finish<<<grid1(n), 256, 0, st>>>(cur, parent, n, out);
             kt_.stop();
