@@ -401,16 +401,17 @@ def separable_taps(sigma, hw):
     tiralib_gb300/csrc/vote3_sep.cu (sep_terms)."""
     text = open(os.path.join(HERE, "tiralib_gb300", "csrc", "vote3_sep_tables.inc")).read()
     num = r"\{([^{}]*)\}"
-    for row in re.finditer(r"\{([\d.]+)f,\s*(\d+),\s*" + r",\s*".join([num] * 4), text):
-        if sigma > float(row[1]):
+    for row in re.finditer(r"\{(\d+),\s*(\d+),\s*" + r",\s*".join([num] * 4), text):
+        if min(3.0 * hw * hw, 104.0 * sigma ** 2) > int(row[1]):
             continue
         b, *w = [[float(v) for v in row[i].split(",") if v.strip()] for i in (3, 4, 5, 6)]
         taps = 0
         for t in range(int(row[2])):
-            h, g = hw, b[t] + 0.5 / sigma ** 2
+            h = hw
             while t > 0 and h > 1:
                 q = float(h * h)
-                if q * g < 3.0 or max(abs(w[k][t]) * q ** (k + 1) for k in range(3)) * np.exp(-g * q) > 1e-7:
+                top = max(abs(w[k][t]) * q ** (k + 1) for k in range(3)) * np.exp(-b[t] * q)
+                if (b[t] + sigma ** -2) * q < 104.0 and (q * b[t] < 3.0 or top > 3e-8):
                     break
                 h -= 1
             taps += 2 * h + 1
