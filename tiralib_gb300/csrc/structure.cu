@@ -728,9 +728,9 @@ int structure_tensor3_device(const float* vol, unsigned s0, unsigned s1, unsigne
     if (tma) {
         fn = tfn;
         smem = tma_smem;
-        TVGB_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
+        TVGB_CUDA(allow_smem(fn, smem));
     } else if (!fixed) {
-        TVGB_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
+        TVGB_CUDA(allow_smem(fn, smem));
     }
     // z chunk.  Each CTA walks zc + K - 1 planes (K - 1 of them ramp).  Cost
     // model: the busiest SM's planes, divided by the speed-up of running n
@@ -935,7 +935,7 @@ int tvgb_structure_tensor2(const float* image, unsigned s0, unsigned s1, float s
     a.img = din.get<float>();
     a.out4 = dout.get<float>();
     const int smem = 4 * st2_smem(int(K));
-    TVGB_CUDA(cudaFuncSetAttribute(k_st2, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+    TVGB_CUDA(allow_smem(k_st2, size_t(smem)));
     dim3 blk(32, 8), grid(ceil_div(a.o1, S2X), ceil_div(a.o0, S2Y));
     {
         KernelTimer kt_("k_st2", st);

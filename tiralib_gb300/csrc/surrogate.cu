@@ -469,7 +469,7 @@ int sur_eval_tc_device(const void* img, const float* X, size_t n, float* Y, int 
     const unsigned grid = unsigned(tiles < 152 * 4 ? tiles : 152 * 4);
     const int smem = TC_SMEM_PER_CTA;
     const void* fn = gelu_mode == 0 ? (const void*)k_sur_eval_tc<0> : (const void*)k_sur_eval_tc<1>;
-    TVGB_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+    TVGB_CUDA(allow_smem(fn, size_t(smem)));
     const uint4* img4 = static_cast<const uint4*>(img);
     void* args[] = {&img4, &X, &n, &Y, &err, &wait_limit};
     {
@@ -522,7 +522,7 @@ static unsigned grid_n(size_t n, unsigned per) {
 static int fwd_bwd_launch(const float* P, const float* X, const float* T, size_t n, size_t first, int batch,
                           float* part, cudaStream_t st) {
     const size_t smem = sizeof(TrainShared);
-    TVGB_CUDA(cudaFuncSetAttribute(k_sur_fwd_bwd, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
+    TVGB_CUDA(allow_smem(k_sur_fwd_bwd, smem));
     {
         KernelTimer kt_("k_sur_fwd_bwd", st);
         k_sur_fwd_bwd<<<batch / TRB, 256, smem, st>>>(P, X, T, n, first, batch, part);

@@ -119,6 +119,19 @@ struct Scratch {
     template <class T> T* get() const { return static_cast<T*>(p); }
 };
 
+// Lets a kernel be launched with `need` bytes of dynamic shared memory.  The
+// limit is one value per kernel and device, and a launch above it fails, so it
+// is always set to the same: with each call setting its own size, a thread
+// that voted a small window between another thread's setting and launch
+// made that launch fail.  226 KB: a CTA's 227 KB less the little static shared
+// memory that some of the kernels have.
+constexpr size_t kMaxDynamicSmem = 226 * 1024;
+template <class F>
+inline cudaError_t allow_smem(F* kernel, size_t need) {
+    if (need > kMaxDynamicSmem) return cudaErrorInvalidValue;
+    return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kMaxDynamicSmem));
+}
+
 inline cudaStream_t as_stream(void* s) { return static_cast<cudaStream_t>(s); }
 
 // Synchronise when any caller array was host memory (its data must be in

@@ -541,7 +541,7 @@ static int vote2_tk_launch(const float4* V, const Nb2* host_or_dev_nb, int nbc, 
             else if (stick) fn = p == 1 ? (const void*)k_vote2_tks<V2R, TY, V2NBC, true, false, true>
                                         : (const void*)k_vote2_tks<V2R, TY, V2NBC, true, false, false>;
             else fn = (const void*)k_vote2_tks<V2R, TY, V2NBC, false, true, true>;
-            TVGB_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem_s)));
+            TVGB_CUDA(allow_smem(fn, smem_s));
             dim3 gs(ceil_div(S1, V2X), ceil_div(S0, unsigned(TY * V2R))), bs(V2X, TY);
             const float4* vp = V;
             const Nb2* tp = dnb.get<Nb2>();
@@ -742,7 +742,7 @@ int tvgb_tensorvote_sweep(const float* t_in, const float* G, unsigned shape0, un
             const size_t smem = sweep_smem(a.set[0].h) * sizeof(float4) <= 110 * 1024 ? 110 * 1024 : 200 * 1024;
             a.stage_floats4 = int(smem / sizeof(float4));
             void (*kern)(SweepArgs) = use_plate ? k_vote2_sweep<true> : k_vote2_sweep<false>;
-            TVGB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
+            TVGB_CUDA(allow_smem(kern, smem));
             {
                 KernelTimer kt_("k_vote2_sweep", st);
                 kern<<<dim3(ceil_div(shape1, V2X), ceil_div(shape0, 32u), unsigned(staged)), dim3(V2X, 8), smem, st>>>(a);

@@ -190,7 +190,7 @@ int vote3_pow_launch(FastArgs f, unsigned power, bool S, bool P, bool B, cudaStr
     const size_t smem = pow_smem(f.hw, rows, S, P, B);
     const dim3 grid(ceil_div(f.s2, PX), ceil_div(f.s1, PY), f.s0), block(PX, PY);
     auto run = [&](auto kern) -> int {
-        TVGB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
+        TVGB_CUDA(allow_smem(kern, smem));
         {
             KernelTimer kt_("k_vote3_pow", st);
             kern<<<grid, block, smem, st>>>(a);
