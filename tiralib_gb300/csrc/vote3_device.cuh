@@ -110,11 +110,14 @@ __device__ __forceinline__ void write_receiver(const FastArgs& a, size_t idx, si
     }
 }
 
-// A volume of fewer than 152 groups of 32 x 8 x 4 receivers, the pair-by-pair
-// kernel's CTA, leaves SMs without one: there it takes one receiver plane per
-// CTA (24 x 20 x 28, sigma 1.5: 76 us instead of 215).
+// A volume of few groups of 32 x 8 x 4 receivers, the pair-by-pair kernel's
+// CTA, leaves SMs without one: there it takes one receiver plane per CTA (24 x
+// 20 x 28, sigma 1.5: 76 us instead of 215).  114 groups are three CTAs of a
+// plane for every SM.  Four planes' time over one's, windows 7 .. 61, with and
+// without the ball: 24 groups 2.6 .. 3.4, 72 1.6 .. 2.0, 100 1.1 .. 1.6, 120
+// 0.99 .. 1.2, 150 0.80 .. 1.10.
 inline bool vote3_small(unsigned planes, unsigned s1, unsigned s2) {
-    return size_t(ceil_div(s2, 32u)) * ceil_div(s1, 8u) * ceil_div(planes, 4u) < 152;
+    return size_t(ceil_div(s2, 32u)) * ceil_div(s1, 8u) * ceil_div(planes, 4u) <= 114;
 }
 
 }  // namespace tvgb
