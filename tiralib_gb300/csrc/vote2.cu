@@ -238,25 +238,31 @@ __global__ void __launch_bounds__(V2X * TY) k_vote2_tks(const float4* __restrict
 
 // ---------------------------------------------------------------- a batch of votes
 // K parameter sets voted on one field in one launch (grid.z: the set), for the
-// parameter sweep.  A CTA of 32 x 8 threads owns 32 x 32 receivers of a set
-// (4 per thread).  It works through the window in bands of offset rows: the
-// band's Neighbor2D entries are computed in place by the CTA's own threads
-// (the steps of build_table; each serves 1024 receivers, so computing it costs
-// under 2% of using it, where the host took ~5 ms for a 121^2 table and the
-// stream waited for its upload), and the voters that the band reaches are
-// staged beside them, so any window up to ~190 pixels runs from shared memory.
-// One launch of all sets fills the SMs that a set of a 160^2 field alone leaves
-// idle (25 CTAs).  45 sets on 160^2, sigma <= 20, powers <= 20: 7.7 ms
-// against 89.7 ms for a launch and, past the kept tables, a host table per set.
+// parameter sweep.  A first launch computes every set's Neighbor2D entries
+// (the steps of build_table) on the device, where the host took ~5 ms for a
+// 121^2 table and the stream waited for its upload.  A CTA of 32 x 8 threads
+// owns 32 x 32 receivers of a set (4 per thread).  It works through the window
+// in bands of offset rows: the band's entries and the voters that the band
+// reaches are staged side by side, so any window up to 347 pixels runs from
+// shared memory.  One launch of all sets fills the SMs that a set of a 160^2
+// field alone leaves idle (25 CTAs).  45 sets on 160^2, sigma <= 20, powers <=
+// 20: 10.2 ms against 118 ms for a launch and, past the kept tables, a host
+// table per set (10.8 with the entries computed by each CTA).  One set of power
+// 1 on 2048^2, sigma 10, 20 and 200 samples: 9.8 ms both, against 12.0 from a
+// kept table, and 12.4 and 16.3 with entries computed by each CTA and one kernel
+// for all powers; sigma 2: 0.86 against 0.88, and 1.02 and 1.27.  The window
+// loop unrolled by 1, 2 and 4, that set: 11.5, 10.5 and 9.8 ms.
 struct SweepSet {
     float s1, s2, eta;
     int h, power, out;        // out: position of the set's field and SIMF
+    int entries;              // position of its first entry
 };
 constexpr int SWEEP_SETS = 128;
 struct SweepArgs {
     const float4* V;
     float4* out;              // + set.out * n
-    int s0, s1, samples, stage_floats4;
+    float4* entries;          // + 2 set.entries
+    int s0, s1, samples;
     SweepSet set[SWEEP_SETS];
 };
 
@@ -298,14 +304,25 @@ __device__ __forceinline__ SweepEntry sweep_entry(const SweepSet& s, int samples
     return e;
 }
 
+template <bool PLATE>
+__global__ void __launch_bounds__(256) k_sweep_entries(const __grid_constant__ SweepArgs a) {
+    const SweepSet& s = a.set[blockIdx.y];
+    const int w = 2 * s.h + 1, i = blockIdx.x * 256 + threadIdx.x;
+    if (i >= w * w) return;
+    const SweepEntry e = sweep_entry(s, a.samples, PLATE, i % w - s.h, i / w - s.h);
+    a.entries[2 * (size_t(s.entries) + i)] = e.a;
+    a.entries[2 * (size_t(s.entries) + i) + 1] = e.b;
+}
+
 template <bool PLATE, bool P1>
-__device__ __forceinline__ void sweep_body(const SweepArgs& a, const SweepSet& s, float4* smem) {
+__device__ __forceinline__ void sweep_body(const SweepArgs& a, const SweepSet& s, float4* smem,
+                                           int stage_floats4) {
     constexpr int VR = 4, TYS = 8, NT = V2X * TYS;
     const int h = s.h, w = 2 * h + 1, TW = V2X + 2 * h;
     const int tid = threadIdx.y * V2X + threadIdx.x;
     const int x0 = blockIdx.x * V2X, y0 = blockIdx.y * (TYS * VR);
     // offset rows per band: entries (2 float4 each) and the voters of TYS VR + rows - 1 rows
-    const int band = min(w, (a.stage_floats4 - (TYS * VR - 1) * TW) / (TW + 2 * w));
+    const int band = min(w, (stage_floats4 - (TYS * VR - 1) * TW) / (TW + 2 * w));
     float4* ent = smem;
     float4* tile = smem + 2 * w * band;
     float sa[VR], sb[VR], sc[VR], pa[VR], pb[VR], pc[VR];
@@ -314,12 +331,8 @@ __device__ __forceinline__ void sweep_body(const SweepArgs& a, const SweepSet& s
     for (int v0 = -h; v0 <= h; v0 += band) {
         const int nb = min(band, h - v0 + 1);
         __syncthreads();                  // the previous band is done with
-        for (int i = tid; i < nb * w; i += NT) {
-            const int dv = i / w, du = i - dv * w;
-            const SweepEntry e = sweep_entry(s, a.samples, PLATE, du - h, v0 + dv);
-            ent[2 * i] = e.a;
-            ent[2 * i + 1] = e.b;
-        }
+        const float4* src = a.entries + 2 * (size_t(s.entries) + size_t(v0 + h) * w);
+        for (int i = tid; i < 2 * nb * w; i += NT) ent[i] = __ldg(src + i);
         for (int i = tid; i < (TYS * VR + nb - 1) * TW; i += NT) {
             const int r = i / TW, c = i - r * TW;
             const int gy = y0 + v0 + r, gx = x0 - h + c;
@@ -330,6 +343,7 @@ __device__ __forceinline__ void sweep_body(const SweepArgs& a, const SweepSet& s
         for (int dv = 0; dv < nb; ++dv) {
             const float4* vrow = tile + (int(threadIdx.y) + dv) * TW + threadIdx.x;
             const float4* erow = ent + 2 * dv * w;
+#pragma unroll 4
             for (int k = 0; k < w; ++k) {
                 const float4 ea = erow[2 * k], eb = erow[2 * k + 1];
                 float4 v[VR];
@@ -389,16 +403,23 @@ __device__ __forceinline__ void sweep_body(const SweepArgs& a, const SweepSet& s
     }
 }
 
-template <bool PLATE>
-__global__ void __launch_bounds__(V2X * 8, 2) k_vote2_sweep(const __grid_constant__ SweepArgs a) {
+// sets first .. first + gridDim.z - 1, all of power 1 (ALL1: 3 CTAs per SM, which the powers' registers do not allow)
+// or of any power
+template <bool PLATE, bool ALL1>
+__global__ void __launch_bounds__(V2X * 8, ALL1 ? 3 : 2) k_vote2_sweep(const __grid_constant__ SweepArgs a, int first,
+                                                                      int stage_floats4) {
     extern __shared__ __align__(16) float4 sm2[];
-    const SweepSet& s = a.set[blockIdx.z];
-    if (s.power == 1) sweep_body<PLATE, true>(a, s, sm2);
-    else sweep_body<PLATE, false>(a, s, sm2);
+    const SweepSet& s = a.set[first + blockIdx.z];
+    if (ALL1 || s.power == 1) sweep_body<PLATE, true>(a, s, sm2, stage_floats4);
+    else sweep_body<PLATE, false>(a, s, sm2, stage_floats4);
 }
 
-// float4s that a band of one row needs; the window rows that fit are taken
-static size_t sweep_smem(int h) { return size_t(32) * (V2X + 2 * h) + 2 * (2 * size_t(h) + 1); }
+// float4s that a band of `rows` window rows needs; the rows that fit are taken
+static size_t sweep_smem(int h, int rows) {
+    return size_t(31 + rows) * (V2X + 2 * h) + 2 * (2 * size_t(h) + 1) * rows;
+}
+constexpr size_t SWEEP_SMEM = 200 * 1024, SWEEP_SMEM2 = 110 * 1024;   // one CTA per SM; two
+constexpr size_t SWEEP_ENTRIES = size_t(8) << 20;                     // of a launch: 256 MB (one set has at most 120409)
 
 // atv (2D, tensorvote.h:225) with atv_H (:161); out [a, b, c]
 __device__ __forceinline__ void atv2_pair(float l0, float l1, float e0x, float e0y, float e1x, float e1y, float rx,
@@ -715,22 +736,27 @@ int tvgb_tensorvote_sweep(const float* t_in, const float* G, unsigned shape0, un
         int w = 2 * int(3.0 * sm) + 1;        // optimize.py:9-15
         if (w < 3) w = 3;
         if (w % 2 == 0) w += 1;
-        sets[k] = SweepSet{float(s1d), float(s2d), stick_norm_2d_h(float(s1d), float(s2d), unsigned(pw)), w / 2, pw, k};
+        sets[k] = SweepSet{float(s1d), float(s2d), stick_norm_2d_h(float(s1d), float(s2d), unsigned(pw)), w / 2, pw, k, 0};
     }
     // widest windows first: they are the longest CTAs
     std::stable_sort(sets.begin(), sets.end(), [](const SweepSet& a, const SweepSet& b) { return a.h > b.h; });
     std::vector<int> row(K);                  // set k's SIMF sums
     const bool use_plate = plate != 0 && samples > 0;
-    for (int k0 = 0; k0 < K; k0 += per) {
-        const int m = std::min(per, K - k0);
+    auto staged_set = [](const SweepSet& s) { return sweep_smem(s.h, 1) * sizeof(float4) <= SWEEP_SMEM; };
+    for (int k0 = 0, m = 0; k0 < K; k0 += m) {
         SweepArgs a{};
         a.V = sv.get<float4>(); a.out = fields; a.s0 = int(shape0); a.s1 = int(shape1); a.samples = int(samples);
         int staged = 0;
-        for (int i = 0; i < m; ++i) {
-            SweepSet s = sets[k0 + i];
-            row[s.out] = t_out ? s.out : k0 + i;
-            if (!t_out) s.out = i;
-            if (sweep_smem(s.h) * sizeof(float4) <= 200 * 1024) {
+        size_t entries = 0;
+        for (m = 0; m < per && k0 + m < K; ++m) {
+            SweepSet s = sets[k0 + m];
+            const size_t ne = staged_set(s) ? size_t(2 * s.h + 1) * (2 * s.h + 1) : 0;
+            if (entries + ne > SWEEP_ENTRIES) break;
+            row[s.out] = t_out ? s.out : k0 + m;
+            if (!t_out) s.out = m;
+            if (ne) {
+                s.entries = int(entries);
+                entries += ne;
                 a.set[staged++] = s;
             } else {                          // a window too wide to stage: a vote by itself, from a table
                 TVGB_TRY(vote2_tk_launch(sv.get<float4>(), nullptr, 0, s.s1, s.s2, s.power, unsigned(2 * s.h + 1), shape0,
@@ -738,17 +764,40 @@ int tvgb_tensorvote_sweep(const float* t_in, const float* G, unsigned shape0, un
             }
         }
         if (staged > 0) {
-            // two CTAs per SM (110 KB) where that holds an offset row of the widest set
-            const size_t smem = sweep_smem(a.set[0].h) * sizeof(float4) <= 110 * 1024 ? 110 * 1024 : 200 * 1024;
-            a.stage_floats4 = int(smem / sizeof(float4));
-            void (*kern)(SweepArgs) = use_plate ? k_vote2_sweep<true> : k_vote2_sweep<false>;
-            TVGB_CUDA(allow_smem(kern, smem));
+            Scratch se;
+            TVGB_TRY(se.alloc(entries * sizeof(SweepEntry), st));
+            a.entries = se.get<float4>();
+            const int wmax = 2 * a.set[0].h + 1;
+            // a set that fills the SMs by itself votes with those of its kind: power 1, or above
+            const unsigned gx = ceil_div(shape1, V2X), gy = ceil_div(shape0, 32u);
+            const auto one = [](const SweepSet& s) { return s.power == 1; };
+            int ones = int(std::count_if(a.set, a.set + staged, one));
+            if (size_t(gx) * gy >= 304) std::stable_partition(a.set, a.set + staged, one);
+            else if (ones < staged) ones = 0;
             {
-                KernelTimer kt_("k_vote2_sweep", st);
-                kern<<<dim3(ceil_div(shape1, V2X), ceil_div(shape0, 32u), unsigned(staged)), dim3(V2X, 8), smem, st>>>(a);
+                KernelTimer kt_("k_sweep_entries", st);
+                auto tab = use_plate ? k_sweep_entries<true> : k_sweep_entries<false>;
+                tab<<<dim3(ceil_div(size_t(wmax) * wmax, 256u), unsigned(staged)), 256, 0, st>>>(a);
                 kt_.stop();
             }
             TVGB_LAUNCHED();
+            auto vote = [&](int first, int count, auto kern) -> int {
+                if (count == 0) return TVGB_OK;
+                // what the widest set's window takes whole, or two CTAs per SM where that holds an offset row of it
+                const int h = a.set[first].h;
+                size_t smem = sweep_smem(h, 2 * h + 1) * sizeof(float4);
+                if (smem > SWEEP_SMEM2) smem = sweep_smem(h, 1) * sizeof(float4) <= SWEEP_SMEM2 ? SWEEP_SMEM2 : SWEEP_SMEM;
+                TVGB_CUDA(allow_smem(kern, smem));
+                {
+                    KernelTimer kt_("k_vote2_sweep", st);
+                    kern<<<dim3(gx, gy, unsigned(count)), dim3(V2X, 8), smem, st>>>(a, first, int(smem / sizeof(float4)));
+                    kt_.stop();
+                }
+                TVGB_LAUNCHED();
+                return TVGB_OK;
+            };
+            TVGB_TRY(vote(0, ones, use_plate ? k_vote2_sweep<true, true> : k_vote2_sweep<false, true>));
+            TVGB_TRY(vote(ones, staged - ones, use_plate ? k_vote2_sweep<true, false> : k_vote2_sweep<false, false>));
         }
         if (!t_out) TVGB_TRY(simf2_device(dG.get<float4>(), fields, n, m, sacc.get<double>() + 3 * size_t(k0), st));
     }
