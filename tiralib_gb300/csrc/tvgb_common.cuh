@@ -109,11 +109,13 @@ struct Scratch {
     Scratch() = default;
     Scratch(const Scratch&) = delete;
     Scratch& operator=(const Scratch&) = delete;
-    ~Scratch() {
+    ~Scratch() { release(); }
+    void release() {
         if (p) {
             cudaFreeAsync(p, stream);
             scratch_track(-(long long)bytes);
         }
+        p = nullptr;
     }
     int alloc(size_t bytes, cudaStream_t s);
     template <class T> T* get() const { return static_cast<T*>(p); }

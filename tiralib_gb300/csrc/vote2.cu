@@ -707,15 +707,8 @@ int tvgb_tensorvote_sweep(const float* t_in, const float* G, unsigned shape0, un
     TVGB_CHECK_ARG(reinterpret_cast<uintptr_t>(din.dev) % 16 == 0 && reinterpret_cast<uintptr_t>(dG.dev) % 16 == 0 &&
                        reinterpret_cast<uintptr_t>(dout.dev) % 16 == 0,
                    "tvgb_tensorvote_sweep: fields must be 16-byte aligned");
-    Scratch sv, sb, sacc;
+    Scratch sv, sacc;
     TVGB_TRY(sv.alloc(n * 16, st));
-    // sets per launch; fields that the caller does not take are kept within 1 GiB
-    int per = std::min(K, SWEEP_SETS);
-    if (!t_out) {
-        per = int(std::max<size_t>(1, std::min<size_t>(per, (size_t(1) << 30) / (n * 16))));
-        TVGB_TRY(sb.alloc(size_t(per) * n * 16, st));
-    }
-    float4* fields = t_out ? dout.get<float4>() : sb.get<float4>();
     TVGB_TRY(sacc.alloc(size_t(K) * 3 * sizeof(double), st));
     int dev = 0, sms = 152;
     cudaGetDevice(&dev);
@@ -742,16 +735,38 @@ int tvgb_tensorvote_sweep(const float* t_in, const float* G, unsigned shape0, un
     std::stable_sort(sets.begin(), sets.end(), [](const SweepSet& a, const SweepSet& b) { return a.h > b.h; });
     std::vector<int> row(K);                  // set k's SIMF sums
     const bool use_plate = plate != 0 && samples > 0;
-    auto staged_set = [](const SweepSet& s) { return sweep_smem(s.h, 1) * sizeof(float4) <= SWEEP_SMEM; };
+    auto entries_of = [](const SweepSet& s) {  // of a set whose window is staged; 0: too wide
+        const size_t w = 2 * size_t(s.h) + 1;
+        return sweep_smem(s.h, 1) * sizeof(float4) <= SWEEP_SMEM ? w * w : size_t(0);
+    };
+    // sets and entries per launch: fields that the caller does not take within 1 GiB, and less of both, down to a set's,
+    // where the device has no more
+    size_t widest = 0, share = 0;
+    for (const SweepSet& s : sets) {
+        widest = std::max(widest, entries_of(s));
+        share = std::min(share + entries_of(s), SWEEP_ENTRIES);
+    }
+    int per = std::min(K, SWEEP_SETS);
+    if (!t_out) per = int(std::max<size_t>(1, std::min<size_t>(per, (size_t(1) << 30) / (n * 16))));
+    Scratch sb, se;
+    for (;; per = (per + 1) / 2, share = std::max(widest, share / 2)) {
+        int rc = t_out ? TVGB_OK : sb.alloc(size_t(per) * n * 16, st);
+        if (rc == TVGB_OK) rc = se.alloc(share * sizeof(SweepEntry), st);
+        if (rc == TVGB_OK) break;
+        sb.release();
+        if (rc != TVGB_ERR_NOMEM || (per == 1 && share == widest)) return rc;
+        cudaGetLastError();
+    }
+    float4* fields = t_out ? dout.get<float4>() : sb.get<float4>();
     for (int k0 = 0, m = 0; k0 < K; k0 += m) {
         SweepArgs a{};
-        a.V = sv.get<float4>(); a.out = fields; a.s0 = int(shape0); a.s1 = int(shape1); a.samples = int(samples);
+        a.V = sv.get<float4>(); a.out = fields; a.entries = se.get<float4>(); a.s0 = int(shape0); a.s1 = int(shape1); a.samples = int(samples);
         int staged = 0;
         size_t entries = 0;
         for (m = 0; m < per && k0 + m < K; ++m) {
             SweepSet s = sets[k0 + m];
-            const size_t ne = staged_set(s) ? size_t(2 * s.h + 1) * (2 * s.h + 1) : 0;
-            if (entries + ne > SWEEP_ENTRIES) break;
+            const size_t ne = entries_of(s);
+            if (entries + ne > share) break;
             row[s.out] = t_out ? s.out : k0 + m;
             if (!t_out) s.out = m;
             if (ne) {
@@ -764,9 +779,6 @@ int tvgb_tensorvote_sweep(const float* t_in, const float* G, unsigned shape0, un
             }
         }
         if (staged > 0) {
-            Scratch se;
-            TVGB_TRY(se.alloc(entries * sizeof(SweepEntry), st));
-            a.entries = se.get<float4>();
             const int wmax = 2 * a.set[0].h + 1;
             // a set that fills the SMs by itself votes with those of its kind: power 1, or above
             const unsigned gx = ceil_div(shape1, V2X), gy = ceil_div(shape0, 32u);
