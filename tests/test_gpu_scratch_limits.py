@@ -1,5 +1,6 @@
 """Calls that need less scratch than they like: with the device nearly full
-the sweep votes fewer sets at a time.  In a process of its own, whose memory is its own."""
+the separable vote takes fewer planes at a time and at last gives way to the
+pair-by-pair one, and the sweep votes fewer sets at a time.  Each in a process of its own, whose memory is its own."""
 import os
 import subprocess
 import sys
@@ -40,7 +41,23 @@ hog = leave(400 << 20)
 np.testing.assert_allclose(np.asarray(optimize.tk_sweep(G, I, params)), want, rtol=1e-10)
 """
 
-@pytest.mark.parametrize("body", [SWEEP], ids=["sweep"])
+VOTE3 = """
+T = torch.rand((160, 192, 192, 6), device="cuda")
+kw = dict(w=25, layout="sym6", out_layout="sym6", parity=False)
+tv.vote3(T[:24].contiguous(), 1.0, w=5, layout="sym6", out_layout="sym6", parity=False)
+(out, _, _), names = kernels_of(lambda: tv.vote3(T, 4.0, **kw))
+assert "k_sep_xy" in names
+for free, kernel, other in (((1200 << 20), "k_sep_xy", "k_vote3_fast"),        # fewer planes at a time
+                            ((500 << 20), "k_vote3_fast", "k_sep_xy")):        # not the 540 MB of moments and votes
+    hog = leave(free)
+    (got, _, _), names = kernels_of(lambda: tv.vote3(T, 4.0, **kw))
+    assert kernel in names and other not in names, names
+    assert float((got - out).abs().max()) <= 1e-5 * float(out.abs().max())
+    del got, hog
+"""
+
+
+@pytest.mark.parametrize("body", [SWEEP, VOTE3], ids=["sweep", "vote3"])
 def test_a_nearly_full_device(body):
     code = CHILD.format(here=HERE, repo=os.path.dirname(HERE), body=body)
     r = subprocess.run([sys.executable, "-c", code], capture_output=True, text=True, timeout=300)
