@@ -231,18 +231,20 @@ __global__ void __launch_bounds__(CT * 8) k_close(const unsigned char* __restric
 // every retry ends.  Three launches and no word from the host; tiles that
 // propagated by rounds, with a synchronisation after each, took 1.2 of the
 // 1.43 ms of a 1024^2 mask.
+//
+// The root of x by path halving (Tarjan and van Leeuwen, 1984): each node on
+// the way is hung on its grandparent.  Other threads write the same nodes, but
+// only ever one of a node's ancestors, and only to nodes that are no roots.
 template <class I>
 __device__ __forceinline__ I uf_find(I* __restrict__ p, I x) {
-    I cur = *static_cast<volatile I*>(p + x);
-    if (cur != x) {
-        I prev = x, next;
-        while (cur > (next = *static_cast<volatile I*>(p + cur))) {   // halve the path: prev is no root, its parent may
-            *static_cast<volatile I*>(p + prev) = next;               // be any of its ancestors
-            prev = cur;
-            cur = next;
-        }
+    volatile I* parent = p;
+    for (;;) {
+        const I up = parent[x];
+        if (up == x) return x;
+        const I top = parent[up];
+        if (top != up) parent[x] = top;
+        x = top;
     }
-    return cur;
 }
 __device__ __forceinline__ unsigned uf_cas(unsigned* a, unsigned c, unsigned v) { return atomicCAS(a, c, v); }
 __device__ __forceinline__ unsigned long long uf_cas(unsigned long long* a, unsigned long long c, unsigned long long v) {
