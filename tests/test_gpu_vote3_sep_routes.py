@@ -1,5 +1,5 @@
 """Ways through the separable 3D vote: host outputs in slabs, a volume cut into
-z-slabs, and second Gaussians of any width."""
+z-slabs, and Gaussians of any width against the window."""
 import numpy as np
 import pytest
 
@@ -57,8 +57,12 @@ def test_z_slabs_of_a_volume(parts):
 
 
 @pytest.mark.parametrize("sigma,sigma2,w", [(2.0, 5.0, 31), (4.0, 0.6, 25), (1.0, 4.0, 0), (3.0, 3.0, 0),
-                                            (3.0, 2.999, 0)])
-def test_second_gaussians(sigma, sigma2, w):
+                                            (3.0, 2.999, 0),
+                                            (10.0, 0.0, 41), (1.0, 0.0, 25), (0.6, 0.0, 21)])
+def test_gaussians_of_any_width(sigma, sigma2, w):
+    """The second Gaussian wider, narrower, equal and nearly so; one Gaussian
+    wider than its window, and windows of 12 and 17 sigma, past which FP32 has
+    no weight left."""
     import torch
     import tiralib_gb300 as tv
     shape = (40, 70, 90)
