@@ -55,7 +55,7 @@ def pipeline3_slab(volume, z0, z1, sigma_st, sigma1, sigma2=0.0, w=0, samples=20
                    evecs="cartesian"):
     """The 3D path for owned planes [z0, z1) of `volume` ((nz, ny, nx), NumPy
     or CUDA torch): (voted planes (6, z1 - z0, ny, nx), eigenvalues,
-    eigenvectors) equal to those planes of the whole-volume result."""
+    eigenvectors): those planes of the whole-volume result, to rounding."""
     from . import api
     nz = int(volume.shape[0])
     (in_lo, in_hi), (st_lo, st_hi) = halo_ranges(nz, z0, z1, sigma_st, sigma1, sigma2, w)
