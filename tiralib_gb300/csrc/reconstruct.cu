@@ -242,7 +242,8 @@ __device__ __forceinline__ I uf_find(I* __restrict__ p, I x) {
         const I up = parent[x];
         if (up == x) return x;
         const I top = parent[up];
-        if (top != up) parent[x] = top;
+        if (top == up) return up;
+        parent[x] = top;
         x = top;
     }
 }
